@@ -1092,6 +1092,9 @@ class Adjoint final : public AdjointBase {
     T* dst[3] = {c0.h, c0.hu, c0.hv};
     for (int k = 0; k < 3; ++k)
       if (upload_interior(dst[k], src[k], 0.0, default_layout()) != 0) return -1;
+    // page-locked arrays are copied after the call returns: the caller may
+    // write or free its arrays only once the copies have ended
+    ADJ_TRY(cudaStreamSynchronize(stream_));
     dts_.assign((size_t)nsteps * nm, 0.0);
     obs_.assign(nres, 0.0);
     mass_.assign(2 * (size_t)nm, 0.0);
