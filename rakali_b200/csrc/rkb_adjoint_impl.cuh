@@ -744,8 +744,9 @@ __device__ __forceinline__ void recon_cell(const Grid& g, const Fields<T>& V,
   gd[3] = db;
 }
 
-// Reconstruction adjoint and slope gather in one launch.  Block (bx, by)
-// gathers the kGX x kGY cells from (ng-2 + bx kGX, ng-2 + by kGY): every cell
+// Reconstruction adjoint and slope gather.  Block (bx, by) of a launch whose
+// first row of blocks is by0 (a launch holds 65535 rows of them) gathers the
+// kGX x kGY cells from (ng-2 + bx kGX, ng-2 + (by0 + by) kGY): every cell
 // collects the slope adjoints of itself and its neighbours (minmod branch a =
 // q_c - q_{c-1}, b = q_{c+1} - q_c), plus the direct reconstruction and
 // cell-update adjoints.  The reconstruction adjoints of the block's cells and
@@ -763,13 +764,13 @@ constexpr int kGX = kRW - 2, kGY = kRH - 2;         // cells it gathers
 template <typename T>
 __global__ void __launch_bounds__(kRN)
     k_recon_gather_adj(Grid g, size_t ms, Fields<T> V, const T* __restrict__ b, Rev<T> R,
-                       Fields<T> gV, T* __restrict__ gb, int frozen, Fields<T> gadd) {
+                       Fields<T> gV, T* __restrict__ gb, int frozen, Fields<T> gadd, int by0) {
   __shared__ T s_gs[6][kRN];
   __shared__ T s_gd[4][kRN];
   __shared__ int s_ch[kRN];
   const int ie = g.nxt - g.ng, je = g.nyt - g.ng;
   const size_t zb = member_base(ms);
-  const int i0 = g.ng - 2 + (int)blockIdx.x * kGX, j0 = g.ng - 2 + (int)blockIdx.y * kGY;
+  const int i0 = g.ng - 2 + (int)blockIdx.x * kGX, j0 = g.ng - 2 + (by0 + (int)blockIdx.y) * kGY;
   // recon cells: [ng-1, ie] x [ng-1, je]
   auto rc = [&](int ii, int jj) { return in_box(ii, jj, g.ng - 1, ie, g.ng - 1, je); };
   {
@@ -1499,11 +1500,14 @@ class Adjoint final : public AdjointBase {
     else
       k_faces_adj<T, false><<<blocks(g_.ng, ie, g_.ng, je), kBX * kBY, 0, stream_>>>(g_, ms_, V,
                                                                                      b_, Tp, R_);
-    const dim3 gather((unsigned)((ie - g_.ng + 4 + kGX - 1) / kGX),
-                      (unsigned)((je - g_.ng + 4 + kGY - 1) / kGY), (unsigned)nm_);
-    k_recon_gather_adj<T><<<gather, kRN, 0,
-                            stream_>>>(g_, ms_, V, b_, R_, gV_, gb_, frozen_ ? 1 : 0,
-                                       stage == 1 ? gbase_ : Fields<T>{});
+    const int rows = (je - g_.ng + 4 + kGY - 1) / kGY;  // of blocks
+    for (int by0 = 0; by0 < rows; by0 += 65535) {
+      const dim3 gather((unsigned)((ie - g_.ng + 4 + kGX - 1) / kGX),
+                        (unsigned)std::min(rows - by0, 65535), (unsigned)nm_);
+      k_recon_gather_adj<T><<<gather, kRN, 0,
+                              stream_>>>(g_, ms_, V, b_, R_, gV_, gb_, frozen_ ? 1 : 0,
+                                         stage == 1 ? gbase_ : Fields<T>{}, by0);
+    }
     walls_adj(V, false);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
   }

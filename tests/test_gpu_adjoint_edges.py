@@ -90,3 +90,31 @@ def test_initial_state_is_taken_by_the_constructor():
             runs.append((J, eta, p.dt, *p.gradient(b, 0.02)))
     for x, y in zip(*runs):
         np.testing.assert_array_equal(x, y)
+
+
+@pytest.mark.parametrize("ny", [393206, 393207, 400001])
+def test_gradient_of_more_rows_than_one_launch_gathers(ny):
+    """65535 blocks of six rows gather the ny + 4 rows up to ny = 393206, beyond
+    it a second launch the rest.  Gauges next to both ends: the gradients there
+    are those of the first and of the last 60 rows alone, and zero between."""
+    from rakali_b200.adjoint import GaugeMisfitBatch
+    nx, m, half = 4, 60, 30  # two steps carry a gauge's gradient 8 rows
+    rng = np.random.default_rng(ny)
+    b = -2.0 + 0.2 * rng.random((1, nx, ny))
+    h, hu = 2.0 + 0.1 * rng.random((1, nx, ny)), rng.normal(0.0, 0.3, (1, nx, ny))
+
+    def gradients(rows, gauges):
+        bp, hp, hup = (np.ascontiguousarray(x[:, :, rows]) for x in (b, h, hu))
+        with GaugeMisfitBatch(1, nx, bp.shape[2], 10.0, 10.0, hp, [gauges], 2, precision=32,
+                              hu0=hup) as p:
+            p.set_dt(np.full((1, 2), 0.5))
+            return p.gradient(bp, 0.02)[1:]
+
+    full = gradients(slice(None), [(1, 3), (2, ny - 4)])
+    low = gradients(slice(0, m), [(1, 3)])
+    high = gradients(slice(ny - m, ny), [(2, m - 4)])
+    for x, lo, hi in zip(full, low, high):
+        assert lo.any() and hi.any()
+        np.testing.assert_array_equal(x[:, :, :half], lo[:, :, :half])
+        np.testing.assert_array_equal(x[:, :, -half:], hi[:, :, -half:])
+        assert not x[:, :, half:-half].any()
