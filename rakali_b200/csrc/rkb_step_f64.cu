@@ -358,12 +358,12 @@ __device__ __forceinline__ void issue_tile(const TileMaps& tm, int in_set, int o
 
 // False when wave_speed(h, u, v) is certain to stay below the maxima already
 // `seen` (x and y), by a single-precision bound on it; true for what is not
-// finite.  The exact speeds (two square roots, two divisions) and the atomics
+// finite, in dry cells too (precipitation and the sponge follow the clamp).  The exact speeds (two square roots, two divisions) and the atomics
 // on the two maxima, which all warps of the grid share, are left to the few
 // warps that may raise them: at 1652 x 1396 the atomics alone, two a warp,
 // held stage 2 at 194 us where stage 1 took 125.
 __device__ __forceinline__ bool outruns(double h, double u, double v, const float* seen) {
-  if (h < kDry) return false;
+  if (h < kDry) return !isfinite(h + u + v);
   const float hf = __double2float_rn(h);
   float rh, c;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rh) : "f"(hf));

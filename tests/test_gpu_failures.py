@@ -109,3 +109,27 @@ def test_nan_in_the_state_is_reported_not_propagated_silently(precision):
         s.step(3)
         assert s.step_count == n0 + 4
         assert np.all(np.isfinite(s.h_phys)) and np.all(np.isfinite(s.hu_phys))
+
+
+@pytest.mark.parametrize("tile", [10, 8])
+@pytest.mark.parametrize("source", ["precipitation", "sponge"])
+def test_an_infinite_negative_depth_is_reported(source, tile):
+    """Depths that terms after the last clamp take to minus infinity: forward
+    Euler adds precipitation there, the sponge relaxes every scheme's depths."""
+    from rakali_b200 import Rakali
+    cfg = dict(nx=NX, ny=NY, dx=DX, dy=DX, t_end=1e6, cfl=0.45)
+    if source == "sponge":  # h - dt alpha (h - h_ref) overflows at the edge
+        cfg.update(bc_west="sponge", sponge_width=8, sponge_strength=100.0, sponge_h_ref=-1.7e308)
+    else:
+        cfg.update(time_scheme="euler")
+    with Rakali(**cfg) as s:
+        s.set_tile(tile)
+        if source == "precipitation":
+            p = np.zeros((NX, NY), order="F")
+            p[70, 31] = -np.inf
+            s.set_precipitation(p)
+        with pytest.raises(RuntimeError, match="non-finite"):
+            s.step(4)
+        assert s.step_count == 1
+        assert np.isneginf(s.h_phys).any()
+        assert not np.isposinf(s.h_phys).any() and not np.isnan(s.h_phys).any()
