@@ -930,7 +930,7 @@ __global__ void k_gauges_adj(const long long* __restrict__ gq, const double* __r
 }
 
 // Host doubles (null: `fill`) -> every cell of a field, ghosts and row padding
-// zero; and the interior back (blockIdx.z: member of this batch of copies).
+// zero; and the interior back (blockIdx.z: member).
 template <typename T>
 __global__ void k_import(Grid g, size_t ms, const double* __restrict__ src, double fill,
                          HostLayout l, T* __restrict__ dst) {
@@ -973,7 +973,6 @@ class Adjoint final : public AdjointBase {
     if (all_mem_) cudaFree(all_mem_);
     if (mem_) cudaFree(mem_);
     if (obs_d_) cudaFree(obs_d_);
-    if (stage_d_) cudaFree(stage_d_);
     if (stream_) cudaStreamDestroy(stream_);
   }
 
@@ -1276,21 +1275,13 @@ class Adjoint final : public AdjointBase {
     return cudaStreamSynchronize(stream_) == cudaSuccess ? 0 : -1;
   }
 
-  // Members of a host field that go through the staging buffer together: all
-  // of them when their values interleave, else as many as fit 64 MB.
-  int staged_members(const HostLayout& l) const {
-    const size_t cells = (size_t)g_.nx_phys() * g_.ny_phys();
-    if (nm_ > 1 && l.m != (long long)cells) return nm_;
-    return (int)std::min<size_t>((size_t)nm_, std::max<size_t>(1, (size_t(64) << 20) / (8 * cells)));
-  }
-  int stage_for(size_t cells) {
-    if (cells <= stage_cells_) return 0;
-    if (stage_d_) cudaFree(stage_d_);
-    stage_d_ = nullptr;
-    stage_cells_ = 0;
-    ADJ_TRY(cudaMalloc((void**)&stage_d_, cells * sizeof(double)));
-    stage_cells_ = cells;
-    return 0;
+  // Where host fields lie on the device on their way in and out: the three
+  // arrays of lam_, which hold nothing outside the reverse sweep (it clears them
+  // first) and follow one another, 12 bytes or more a cell.  No memory is
+  // allocated for it, whatever the order of a batched field's axes.
+  double* staging() const { return (double*)lam_.h; }
+  size_t host_bytes() const {
+    return (size_t)nm_ * g_.nx_phys() * g_.ny_phys() * sizeof(double);
   }
   HostLayout default_layout() const {
     return HostLayout{(long long)g_.nx_phys() * g_.ny_phys(), 1, g_.nx_phys()};
@@ -1300,33 +1291,19 @@ class Adjoint final : public AdjointBase {
   // zero).  The block of doubles goes to the device as it lies; a kernel
   // converts it and lays it out.
   int upload_interior(T* dst, const double* src, double fill, const HostLayout& l) {
-    const size_t cells = (size_t)g_.nx_phys() * g_.ny_phys();
-    const int per = staged_members(l);
-    if (src && stage_for(per * cells) != 0) return -1;
-    for (int m = 0; m < nm_; m += per) {
-      const int n = std::min(per, nm_ - m);
-      if (src)
-        ADJ_TRY(cudaMemcpyAsync(stage_d_, src + (size_t)m * cells, n * cells * sizeof(double),
-                                cudaMemcpyHostToDevice, stream_));
-      const dim3 grid((unsigned)((g_.pitch + 127) / 128), (unsigned)std::min(g_.nyt, 65535), (unsigned)n);
-      k_import<T><<<grid, 128, 0, stream_>>>(g_, ms_, src ? stage_d_ : nullptr, fill, l,
-                                             dst + (size_t)m * ms_);
-    }
+    if (src)
+      ADJ_TRY(cudaMemcpyAsync(staging(), src, host_bytes(), cudaMemcpyHostToDevice, stream_));
+    const dim3 grid((unsigned)((g_.pitch + 127) / 128), (unsigned)std::min(g_.nyt, 65535),
+                    (unsigned)nm_);
+    k_import<T><<<grid, 128, 0, stream_>>>(g_, ms_, src ? staging() : nullptr, fill, l, dst);
     return cudaGetLastError() == cudaSuccess ? 0 : -1;
   }
 
   int download_interior(double* dst, const T* src, const HostLayout& l) {
-    const size_t cells = (size_t)g_.nx_phys() * g_.ny_phys();
-    const int per = staged_members(l);
-    if (stage_for(per * cells) != 0) return -1;
-    for (int m = 0; m < nm_; m += per) {
-      const int n = std::min(per, nm_ - m);
-      const dim3 grid((unsigned)((g_.nx_phys() + 127) / 128),
-                      (unsigned)std::min(g_.ny_phys(), 65535), (unsigned)n);
-      k_export<T><<<grid, 128, 0, stream_>>>(g_, ms_, src + (size_t)m * ms_, l, stage_d_);
-      ADJ_TRY(cudaMemcpyAsync(dst + (size_t)m * cells, stage_d_, n * cells * sizeof(double),
-                              cudaMemcpyDeviceToHost, stream_));
-    }
+    const dim3 grid((unsigned)((g_.nx_phys() + 127) / 128),
+                    (unsigned)std::min(g_.ny_phys(), 65535), (unsigned)nm_);
+    k_export<T><<<grid, 128, 0, stream_>>>(g_, ms_, src, l, staging());
+    ADJ_TRY(cudaMemcpyAsync(dst, staging(), host_bytes(), cudaMemcpyDeviceToHost, stream_));
     return cudaStreamSynchronize(stream_) == cudaSuccess ? 0 : -1;
   }
 
@@ -1544,8 +1521,6 @@ class Adjoint final : public AdjointBase {
   T *b_ = nullptr, *nf_ = nullptr, *gb_ = nullptr, *gn_ = nullptr;
   double* r_ = nullptr;
   double* obs_d_ = nullptr;
-  double* stage_d_ = nullptr;  // host fields on their way in or out
-  size_t stage_cells_ = 0;
   HostLayout lay_b_{}, lay_n_{}, lay_g_{};
   double* dts_d_ = nullptr;
   double* mass_d_ = nullptr;

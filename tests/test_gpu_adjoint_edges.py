@@ -118,3 +118,32 @@ def test_gradient_of_more_rows_than_one_launch_gathers(ny):
         np.testing.assert_array_equal(x[:, :, :half], lo[:, :, :half])
         np.testing.assert_array_equal(x[:, :, -half:], hi[:, :, -half:])
         assert not x[:, :, half:-half].any()
+
+
+@pytest.mark.parametrize("precision", [64, 32])
+def test_fields_in_any_order_take_no_device_memory_of_their_own(precision):
+    """Members that interleave in memory (Fortran order) go through the
+    problem's own arrays: the calls leave the free device memory as it was."""
+    import torch
+
+    from rakali_b200.adjoint import GaugeMisfitBatch
+
+    def problem(nm, nx, ny):
+        rng = np.random.default_rng(nx)
+        b = np.asfortranarray(-2.0 + 0.3 * rng.random((nm, nx, ny)))
+        n = np.asfortranarray(0.02 + 0.01 * rng.random((nm, nx, ny)))
+        return b, n, GaugeMisfitBatch(nm, nx, ny, 10.0, 10.0, 0.1 * rng.random(b.shape) - b,
+                                      [[(3, 4), (9, 11)]] * nm, 2, precision=precision)
+
+    b, n, p = problem(2, 20, 18)  # the library's kernels are loaded by their first use
+    p.record_dt(b, n)
+    p.gradient(b, n)
+    p.close()
+    b, n, p = problem(10, 1024, 1024)  # 84 MB a field on the host
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    p.record_dt(b, n)
+    p.gradient(b, n)
+    p.forward(np.ascontiguousarray(b), n)
+    assert free - torch.cuda.mem_get_info()[0] < 8 << 20  # the observations take a page
+    p.close()
