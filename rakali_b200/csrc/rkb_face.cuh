@@ -10,6 +10,8 @@
 // the B200 kernels evaluate each face once and share it through shared memory.
 #pragma once
 
+#include <type_traits>
+
 #include "rkb_common.cuh"
 #include "rkb_rnmath.cuh"
 
@@ -298,13 +300,19 @@ __device__ __noinline__ void face_general(const double* th, int nt, int q, int d
 
 // Value x + side * minmod(a, b) / 2 of one side of a face (rki_kernel_flux.F90:
 // 159-181, :380-393) for moderate() values: a b <= 0 is a difference of signs
-// (a zero is the smaller of the two anyway), and halving is exact, so the sum
-// rounds once and is one FMA.  The FP64 pipe binds the stage: the sign test and
-// the choice of the factor run beside it.
+// or a zero, and halving is exact, so the sum rounds once and is one FMA.  The
+// FP64 pipe binds the stage: the test runs beside it, on the high words
+// (differences of moderate values are zero or far above the subnormals).
+// ZEROS: x may be -0 (a momentum at rest), and the half-slope that is added or
+// subtracted then has to be +0.  A surface h + b of a wet cell is never -0, and
+// neither the factor's nor the smaller difference's sign matters beside it.
+template <bool ZEROS>
 __device__ __forceinline__ double limited(double x, double a, double b, double side) {
   const double m = fabs(a) < fabs(b) ? a : b;
-  const bool same = (__double2hiint(a) ^ __double2hiint(b)) >= 0;
-  return __fma_rn(same ? 0.5 * side : 0.0, m, x);
+  const int signs = __double2hiint(a) ^ __double2hiint(b);
+  if (!ZEROS) return __fma_rn(signs >= 0 ? 0.5 * side : 0.0, m, x);
+  const int same = (signs & (int)0x80000000) | (__double2hiint(m) & 0x7fffffff);
+  return __fma_rn(0.5 * side, same > 0 ? m : 0.0, x);
 }
 
 // Above a positive threshold for certain (values next to it may say no);
@@ -325,15 +333,17 @@ __device__ __forceinline__ void face_of_tile(const double* th, int nt, int q, in
       clear_of(min(__double2hiint(hm), __double2hiint(hp)), kDry)) {
     const double bL = tb[q], bR = tb[q + d];
     // reconstructed value of both sides of the face
-    auto sides = [](double m, double l, double r, double p, double& vl, double& vr) {
+    auto sides = [](auto zeros, double m, double l, double r, double p, double& vl, double& vr) {
       const double a = l - m, b = r - l, c = p - r;
-      vl = limited(l, a, b, 1.0);
-      vr = limited(r, b, c, -1.0);
+      vl = limited<decltype(zeros)::value>(l, a, b, 1.0);
+      vr = limited<decltype(zeros)::value>(r, b, c, -1.0);
     };
+    const std::false_type surface;
+    const std::true_type momentum;
     double eL, uL, vL, eR, uR, vR;
-    sides(hm + tb[q - d], hL + bL, hR + bR, hp + tb[q + 2 * d], eL, eR);
-    sides(tu[q - d], tu[q], tu[q + d], tu[q + 2 * d], uL, uR);
-    sides(tv[q - d], tv[q], tv[q + d], tv[q + 2 * d], vL, vR);
+    sides(surface, hm + tb[q - d], hL + bL, hR + bR, hp + tb[q + 2 * d], eL, eR);
+    sides(momentum, tu[q - d], tu[q], tu[q + d], tu[q + 2 * d], uL, uR);
+    sides(momentum, tv[q - d], tv[q], tv[q + d], tv[q + 2 * d], vL, vR);
     FaceOut o;
     if (face_flux_wet<DIR, HLLC>(eL, uL, vL, bL, eR, uR, vR, bR, o)) {
       f[0] = o.fh;

@@ -143,3 +143,42 @@ def test_steps_with_extreme_values(kind, hllc, tile):
             orc.step(2)
             assert sim.dt == orc.dt
             compare_state(sim, orc, rtol=0.0)
+
+
+@pytest.mark.parametrize("tile", [10, 8])
+@pytest.mark.parametrize("hllc", [False, True])
+@pytest.mark.parametrize("kind", ["rest", "hump", "rows", "patches"])
+def test_zeros_keep_their_sign(kind, hllc, tile):
+    """Momenta that are zeros of both signs, at rest, beside a hump, across a
+    one-dimensional flow and between moving cells: the oracle's bit patterns
+    (a wall ghost negates, so a lake at rest has zeros of both signs too)."""
+    nx, ny = 53, 41
+    rng = np.random.default_rng(9)
+    h = np.full((nx, ny), 2.0, order="F")
+    hu, hv = (rng.choice([0.0, -0.0], (nx, ny)) for _ in range(2))
+    if kind == "hump":
+        h[20:25, 20:25] = 2.5
+        hv[:], hu[:] = 0.0, 0.0
+        hv[:, ::2], hu[::2] = -0.0, -0.0
+    elif kind == "rows":
+        h[:] = 2.0 + 0.3 * rng.random((nx, 1))
+        hu[:] = rng.normal(0.0, 0.3, (nx, 1))
+    elif kind == "patches":
+        h[:] = 2.0 + 0.3 * rng.random((nx, ny))
+        moving = rng.random((nx, ny)) < 0.3
+        hu[moving] = rng.choice([0.5, -0.5], moving.sum())
+        hv[moving] = rng.choice([0.3, -0.3], moving.sum())
+    cfg = dict(nx=nx, ny=ny, dx=10.0, dy=7.0, t_end=1.0e9, cfl=0.45, manning_n=0.03, use_hllc=hllc)
+    for steps in (1, 3):
+        sim, orc = pair(cfg, bathymetry=np.zeros((nx, ny), order="F"), initial_h=h)
+        with sim:
+            sim.set_tile(tile)
+            for name, f in (("hu", hu), ("hv", hv)):
+                getattr(sim, f"set_{name}")(np.asfortranarray(f))
+                orc.interior(name)[:] = f
+            sim.step(steps)
+            orc.step(steps)
+            for name in ("h", "hu", "hv"):
+                got, want = (np.ascontiguousarray(x).view(np.int64)
+                             for x in (getattr(sim, name), orc.arrays[name]))
+                np.testing.assert_array_equal(got, want)
