@@ -453,7 +453,7 @@ def run_ensemble(args, world, local_rank, dist):
                 ms = ens.time_steps(args.ensemble_steps)
             ms = rp.max_over_ranks(ms, dist)
             # the same steps launch by launch, with events between the phases:
-            # what the six launches of a step cost beyond their kernels
+            # what the launches of a step cost beyond their kernels
             phases = ens.profile_steps(20)
             kernel_sum = sum(phases[k] for k in ("bc_stage1", "stage1", "bc_stage2", "stage2"))
             graph_ms = ms / args.ensemble_steps

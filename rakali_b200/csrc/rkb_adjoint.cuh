@@ -378,10 +378,11 @@ RKB_HD void friction(T h, T& u, T& v, T n, T dt) {
 
 // Adjoint of friction at input (h, u, v, n): (gu, gv) output adjoints in,
 // input adjoints out; gh, gn accumulated.
-// The quotients share one reciprocal per denominator (h, h^(1/3), den, sp),
-// and h^(1/3) is the math library's cube root rather than the correctly
-// rounded one of the forward step: here they only scale adjoints, and no
-// branch depends on them.
+// The quotients share one reciprocal per denominator (h, h^(1/3), den, sp):
+// here they only scale adjoints, and no branch depends on them.  For the same
+// reason GeneralMath takes the math library's cube root, where the forward
+// step's is correctly rounded; WetMath has that one, and its reciprocal comes
+// with it.
 template <typename M = GeneralMath, typename T>
 RKB_HD void friction_adj(T h, T u, T v, T n, T dt, T& gh,
                          T& gu, T& gv, T& gn) {

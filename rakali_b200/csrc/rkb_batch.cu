@@ -375,7 +375,7 @@ int Batch::profile_steps(int n, double out[5]) {
   return finish();
 }
 
-// Candidate shapes: FP64 the four shared-memory tiles; FP32 2 or 4 columns
+// Candidate shapes: FP64 the nine shared-memory tiles; FP32 2 or 4 columns
 // per lane times rows per warp sweep (0 = one wave of resident warps per member).
 int Batch::autotune(int trial_steps, double* best_ms) {
   if (trial_steps <= 0) trial_steps = 3;

@@ -1250,8 +1250,19 @@ static int auto_rows_t(const Grid& g) {
 }
 
 // Least rows for the members of a batch, which share the wave: its strips' rows
-// over the resident warps, from 4 to 16 (20 members of 64^2 .. 1024^2: 16 rows
-// 336 us per step, 8 rows 340, 24 343, 64 405).
+// over the resident warps, from 4 to 16.  us per step, sides uniform in the range:
+//
+//   members, sides       this rule      4      8     16     32     64 rows
+//   4, 64 .. 128              44       45     59     89    155    283
+//   16, 128 .. 256            65       79     74     99    146    271
+//   40, 64 .. 256             93      115    121    118    170    283
+//   20, 64 .. 1024           329      380    336    330    371    386
+//   64, 64 .. 512            365      413    369    366    401    474
+//   4, 1000 .. 1024          253      302    263    253    246    305
+//   256, 64 .. 1024         3966     5041   4313   3963   3839   3843
+//
+// (Large batches gain 3% from 32 rows, which the autotuner finds; smaller ones
+// lose more than that to the warps that 32 rows leave idle.)
 int batch_rows32(const Grid* const* grids, int n, int cpl) {
   long long total = 0;
   for (int k = 0; k < n; ++k) {

@@ -2,7 +2,7 @@
 //
 // A step reads its clock from the device-side StepCtl, so a whole chunk of
 // steps can be captured once in a CUDA graph.  On a grid with free_edges() it is
-// four launches:
+// four launches (three up to 1024 tiles, which one close kernel sums):
 //
 //   stage<1>            U^n -> U*                rki_kernel_flux.F90 + rki_kernel_fused.F90:164-303
 //   stage<2>            U*, U^n -> U^{n+1}       rki_kernel_fused.F90:305-471
@@ -13,7 +13,8 @@
 // cells in memory are filled once, after the run's last step.  Where something
 // reads the ghosts between steps (gauges), or the fills depend on one another
 // (nested and Chapman edges, narrow grids), fills are launches of their own
-// before each stage.
+// before each stage; the marching tiles also take them so, and close the step
+// in stage 2.
 //
 // The CFL reduction (rki_kernel_timestep.F90:16-74) is folded into the
 // stage-2 epilogue; the close turns it into the next step's dt.
@@ -1242,9 +1243,9 @@ static cudaError_t launch_stage_t(const StepArgs& a, FluxOut fl, cudaStream_t s,
 // The TMA-staged kernel: one block per tile.  On a grid of at most two tiles an
 // SM every block has its SM almost to itself, and the time is the length of
 // one warp's chain of dependent FP64 operations, so the blocks are doubled and
-// the two faces of a thread go to two threads: 200 x 100 (84 tiles) 23.4 -> 19.9
-// us a step, 256 x 270 (288) 26.8 -> 24.1.  Two blocks of 512 threads fit an SM,
-// so more tiles than that would wait for a second wave.  (Launching each kernel
+// the two faces of a thread go to two threads: 200 x 100 (91 tiles) 23.4 -> 19.9
+// us a step, 256 x 270 (288) 26.8 -> 24.1.  Two blocks of 512 threads fit each of
+// the B200's 148 SMs, so more tiles than that would wait for a second wave.  (Launching each kernel
 // while the one before still runs, by programmatic dependent launch, came to
 // the same time: 20.5 and 23.5 us.)
 constexpr unsigned kSplitTiles = 2 * 148;
