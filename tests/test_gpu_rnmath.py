@@ -121,6 +121,13 @@ def _state(kind, shape, rng):
     return tuple(np.asfortranarray(x) for x in (h, hu, hv))
 
 
+def _same_bits(sim, orc):
+    for name in ("h", "hu", "hv"):
+        got, want = (np.ascontiguousarray(x).view(np.int64)
+                     for x in (getattr(sim, name), orc.arrays[name]))
+        np.testing.assert_array_equal(got, want)
+
+
 @pytest.mark.parametrize("tile", [10, 8])
 @pytest.mark.parametrize("hllc", [False, True])
 @pytest.mark.parametrize("kind", ["tiny", "still", "thin", "ones", "fast", "huge"])
@@ -143,6 +150,7 @@ def test_steps_with_extreme_values(kind, hllc, tile):
             orc.step(2)
             assert sim.dt == orc.dt
             compare_state(sim, orc, rtol=0.0)
+            _same_bits(sim, orc)
 
 
 @pytest.mark.parametrize("tile", [10, 8])
@@ -178,7 +186,4 @@ def test_zeros_keep_their_sign(kind, hllc, tile):
                 orc.interior(name)[:] = f
             sim.step(steps)
             orc.step(steps)
-            for name in ("h", "hu", "hv"):
-                got, want = (np.ascontiguousarray(x).view(np.int64)
-                             for x in (getattr(sim, name), orc.arrays[name]))
-                np.testing.assert_array_equal(got, want)
+            _same_bits(sim, orc)
